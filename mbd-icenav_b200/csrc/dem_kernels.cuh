@@ -2664,9 +2664,10 @@ __device__ __forceinline__ void resident_step(const KArgs<T>& a, const Frame<T>&
             const T vm = sqrt_nr(v2, h);
             const T vq = q_drag * (vm * vm);
             fd = div_nr(vr, vm, rcp_nr(vm)) * vq;
-            const bool fast = v2 >= FastRange<T>::lo() && vm > T(1e-6);
-            if (!fast) fd = (q_drag * a.fc.lin) * vr;  // too slow (or NaN): linear
-            if (fast && !(v2 <= FastRange<T>::hi() && fast_num(vr))) {
+            // beyond the fast range, where sqrt_nr has no value, the operators decide
+            const bool over = v2 > FastRange<T>::hi(), quad = over || (v2 >= FastRange<T>::lo() && vm > T(1e-6));
+            if (!quad) fd = (q_drag * a.fc.lin) * vr;  // too slow (or NaN): linear
+            if (quad && (over || !fast_num(vr))) {
                 const T ve_m = jsqrt(v2);
                 fd = (vr / ve_m) * (q_drag * (ve_m * ve_m));
             }
