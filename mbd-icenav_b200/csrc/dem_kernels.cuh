@@ -951,13 +951,19 @@ __device__ void phase_escape(const KArgs<T>& a, const Frame<T>& F, unsigned cnt,
     }
 }
 
+// Whether so many elements escaped (a handle's first call, a call from another
+// state) that every list is rebuilt, by the escape and build_all phases, instead
+// of the marked ones.
+template <typename T>
+__device__ __forceinline__ bool rebuild_all(const KArgs<T>& a, unsigned cnt) {
+    return (unsigned long long)cnt * 8ull > (unsigned long long)a.n;
+}
 // List upkeep at the frame's start (see the notes on the Verlet lists): whether
-// this frame's escapes are processed beside the ship contact.  When most
-// elements escaped (a handle's first call) the escape and build_all phases of
-// substep 0 rebuild every list instead.
+// this frame's escapes are processed beside the ship contact; when every list is
+// rebuilt, that is done before substep 0.
 template <typename T>
 __device__ __forceinline__ bool upkeep_now(const KArgs<T>& a, unsigned cnt) {
-    return cnt != 0u && !((unsigned long long)cnt * 8ull > (unsigned long long)a.n);
+    return cnt != 0u && !rebuild_all(a, cnt);
 }
 
 // Near phase: mark and re-reference the frame's escaped elements.  A few take
@@ -2903,6 +2909,16 @@ __device__ __forceinline__ int resident_ctas(int na) {
     constexpr int kWarps = kThreads / 32;
     return min((int)gridDim.x, max(min((na + 3) / 4, (int)gridDim.x / 2), (na + kWarps - 1) / kWarps));
 }
+// Whether those CTAs are enough to rebuild every list too, where that comes first;
+// with no active element there is none of them.  A one-frame call that rebuilds
+// 12,127 lists takes 210 to 236 us with 100 to 296 such CTAs against 235 to 247
+// phase by phase on the whole grid, 298 against 246 with 50 and 5.8 ms against 0.24
+// with one; 236,640 lists take 770 us with 296 CTAs against 730, 33 ms with four.
+constexpr int kBuildPerCta = 128;
+template <typename T>
+__device__ __forceinline__ bool enough_to_build(const KArgs<T>& a, int na) {
+    return a.n <= kBuildPerCta * resident_ctas(na);
+}
 // Whether the CTAs without one are enough to take those writes: a quarter of the grid.
 __device__ __forceinline__ bool others_write(int na) { return 4 * ((int)gridDim.x - resident_ctas(na)) >= (int)gridDim.x; }
 
@@ -3000,7 +3016,7 @@ __device__ __forceinline__ bool resident_substeps(const KArgs<T>& a, const Frame
     unsigned cnt = ctl.esc;
     for (int s = 0; s < a.k_sub; ++s) {
         const unsigned round = a.round_base + (unsigned)(F.f * a.k_sub + s) + 1u;
-        const bool all = (unsigned long long)cnt * 8ull > (unsigned long long)a.n;
+        const bool all = rebuild_all(a, cnt);
         if (cnt != 0u) {  // uniform over the CTAs
             phase_escape(a, F, cnt, s, round, all, n_cta);
             __syncthreads();
@@ -3275,7 +3291,8 @@ __global__ void __launch_bounds__(kThreads, DEM_MIN_BLOCKS) dem_frames_kernel(co
         } else if (p == per_frame - 1) {
             phase_fracture(a, F, T(ctl.scale), ctl.fb, ctl.act, resident && others_write(ctl.act));
         } else if (p == 4 && persistent && a.force_split != DEM_SPLIT_THREAD &&
-                   ctl.act <= (int)gridDim.x * res_elems<T>()) {
+                   ctl.act <= (int)gridDim.x * res_elems<T>() &&
+                   (!rebuild_all(a, ctl.esc) || enough_to_build(a, ctl.act))) {
             // the CTAs' shared memory holds every active element: all substeps in one go
             if (!resident_substeps(a, F, ph, ctl, smem_raw, &sync, end_phase, mark)) return;
             ph += 3 * k - 1;  // the last force phase has ended
@@ -3285,7 +3302,7 @@ __global__ void __launch_bounds__(kThreads, DEM_MIN_BLOCKS) dem_frames_kernel(co
             const int s = (p - 4) / 3;
             const int sub = (p - 4) % 3;
             const unsigned cnt = ctl.esc;
-            const bool all = (unsigned long long)cnt * 8ull > (unsigned long long)a.n;
+            const bool all = rebuild_all(a, cnt);
             // stamp of this rebuild round, unique since the dirty stamps were last cleared
             const unsigned round = a.round_base + (unsigned)(f * k + s) + 1u;
             if (sub == 0) {
