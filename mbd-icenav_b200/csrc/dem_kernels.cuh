@@ -367,20 +367,28 @@ __device__ bool grid_barrier(const KArgs<T>& a, int next_ph, PhaseCtl* ctl) {
 // barriers of parity 0 and 1.  No CTA can be two barriers ahead, so a field
 // stands still while its barrier's CTAs read it; base holds its last value.
 // The word that ends the wait thus says whether the escape counters need
-// reading at all: a load less on every substep's critical path (0.4 us).
+// reading at all: a load less on every substep's critical path (0.4 us).  In a
+// call of so many substeps that a count could carry into the next bits (sub_flags
+// is 0) none is added, and the counters are always read.
 // Returns 0, 1 (read the counters) or -1 (the wait ran out).
 struct SubSync {
     unsigned long long base[2];
     int flag, res;
 };
 
+// What a CTA of a barrier's n adds to the word.
+__host__ __device__ __forceinline__ unsigned long long sub_arrival(bool first, unsigned n, int parity, bool escape,
+                                                                   bool counted) {
+    const unsigned long long add = (first ? 2048ull - (n - 1u) : 1ull) << 52;
+    return add + (escape && counted ? 1ull << (parity ? 26 : 0) : 0ull);
+}
+
 template <typename T>
 __device__ int sub_barrier(const KArgs<T>& a, unsigned n, int parity, SubSync* y) {
     __syncthreads();
     if (threadIdx.x == 0) {
         const int sh = parity ? 26 : 0;
-        unsigned long long add = (blockIdx.x == 0 ? 2048ull - (n - 1u) : 1ull) << 52;
-        if (y->flag) add += 1ull << sh;
+        const unsigned long long add = sub_arrival(blockIdx.x == 0, n, parity, y->flag != 0, a.sub_flags != 0);
         y->flag = 0;
         const unsigned long long old = atom_add_release_u64(a.sub_bar, add);
         unsigned long long now, t0 = 0;
