@@ -63,6 +63,17 @@ def error_flag(device) -> ErrorFlag:
     return _err(device)
 
 
+def _start_rows(name, M, N, start, start_row):
+    """What the start of M rows' N accumulators has to be."""
+    torch = _tm()
+    if start.dtype != torch.float32 or start.stride(1) != 1 or start.shape[1] < N or (
+            start_row is None and start.shape[0] < M):
+        raise ValueError(f"{name}: start must be fp32 rows of at least N entries with unit column stride")
+    if start_row is not None and (start_row.dtype != torch.int32 or not start_row.is_contiguous()
+                                  or start_row.numel() < M):
+        raise ValueError(f"{name}: start_row must hold M contiguous int32 rows")
+
+
 def gemm(A, B, out=None, bias=None, relu=False, mask=None, out_dtype=None, start=None, start_row=None):
     """``act(A @ B.T + bias) * (mask > 0)`` on the tensor cores.  A (M, K) and B
     (N, K) bf16 with unit column stride (row strides multiples of 8); out (M, N)
@@ -86,12 +97,7 @@ def gemm(A, B, out=None, bias=None, relu=False, mask=None, out_dtype=None, start
     if mask is not None and (mask.dtype != torch.bfloat16 or mask.stride(1) != 1):
         raise ValueError("gemm: mask must be bf16 with unit column stride")
     if start is not None:
-        if start.dtype != torch.float32 or start.stride(1) != 1 or start.shape[1] < N or (
-                start_row is None and start.shape[0] < M):
-            raise ValueError("gemm: start must be fp32 rows of at least N entries with unit column stride")
-        if start_row is not None and (start_row.dtype != torch.int32 or not start_row.is_contiguous()
-                                      or start_row.numel() < M):
-            raise ValueError("gemm: start_row must hold M contiguous int32 rows")
+        _start_rows("gemm", M, N, start, start_row)
         _check(lib().sg_gemm_from(M, N, K, _p(A), A.stride(0), _p(B), B.stride(0), _p(out), out.stride(0), dt, _p(bias),
                                   1 if relu else 0, _p(mask), mask.stride(0) if mask is not None else 0, _p(start),
                                   _p(start_row), start.stride(0), _p(_err(A.device).t), _stream(A)), "sg_gemm_from")
@@ -102,11 +108,23 @@ def gemm(A, B, out=None, bias=None, relu=False, mask=None, out_dtype=None, start
     return out
 
 
+def _operands(name, *ts):
+    """What every tensor-core operand has to be."""
+    bf16 = _tm().bfloat16
+    for t in ts:
+        if t.dtype != bf16 or t.stride(-1) != 1:
+            raise ValueError(f"{name}: operands must be bf16 with unit column stride")
+
+
 def weight_grads(layers):
     """For every (dy, x, g, gb) of ``layers``, in one launch: g (N, K) fp32 = dy.T @ x
     and gb (N,) fp32 = column sums of dy, for dy (R, N) and x (R, K) bf16."""
+    torch = _tm()
     arr = (_abi.SgWeightGrad * len(layers))()
     for q, (dy, x, g, gb) in zip(arr, layers):
+        _operands("weight_grads", dy, x)
+        if g.dtype != torch.float32 or gb.dtype != torch.float32 or not gb.is_contiguous():
+            raise ValueError("weight_grads: g and gb must be fp32, gb contiguous")
         q.R, q.N = dy.shape
         q.K = x.shape[1]
         if x.shape[0] != q.R or tuple(g.shape) != (q.N, q.K) or not g.is_contiguous() or gb.numel() != q.N:
@@ -131,38 +149,65 @@ def conv_forward(x, layers):
     """A stack of 3x3 stride-2 convolutions with ReLU on x (P, S, S, C) bf16, in one
     call (``sg_conv_forward``): ``layers`` holds (w, bias, cols, act) per layer, cols
     and act contiguous bf16 of ``im2col``'s and ``gemm``'s shapes."""
-    P, s, _, cin = x.shape
+    torch = _tm()
+    bf16, f32 = torch.bfloat16, torch.float32
+    P, s, width, cin = x.shape
+    if width != s or x.dtype is not bf16 or not x.is_contiguous():
+        raise ValueError("conv_forward: x (P, S, S, C) must be contiguous bf16")
     arr = (_abi.SgConvLayer * len(layers))()
+    size = s
     for q, (w, bias, cols, act) in zip(arr, layers):
         s //= 2
-        if w.shape[1] != cols.shape[1] or cols.shape[0] != P * s * s or tuple(act.shape) != (cols.shape[0], w.shape[0]):
+        cout, kpad = w.shape
+        ldw, unit = w.stride()
+        rows = P * s * s
+        if cols.shape != (rows, kpad) or act.shape != (rows, cout):
             raise ValueError("conv_forward: cols (P s s, kpad) and act (P s s, cout) of w (cout, kpad) are needed")
-        q.cin, q.cout, q.kpad, q.ldw = cin, w.shape[0], w.shape[1], w.stride(0)
+        if not (w.dtype is bf16 and cols.dtype is bf16 and act.dtype is bf16 and bias.dtype is f32 and unit == 1 and
+                cols.is_contiguous() and act.is_contiguous()):
+            raise ValueError("conv_forward: w, cols and act must be bf16, bias fp32, cols and act contiguous, "
+                             "w with unit column stride")
+        q.cin, q.cout, q.kpad, q.ldw = cin, cout, kpad, ldw
         q.w, q.bias, q.cols, q.act = w.data_ptr(), bias.data_ptr(), cols.data_ptr(), act.data_ptr()
-        cin = q.cout
-    _check(lib().sg_conv_forward(P, x.shape[1], x.data_ptr(), len(layers), arr, _p(_err(x.device).t), _stream(x)),
+        cin = cout
+    _check(lib().sg_conv_forward(P, size, x.data_ptr(), len(layers), arr, _p(_err(x.device).t), _stream(x)),
            "sg_conv_forward")
 
 
 def dense_forward(x, layers):
     """A stack of dense layers on x (R, K) bf16, in one call (``sg_dense_forward``):
-    ``layers`` holds ``gemm``'s (w, bias, relu, out, start, start_row) per layer."""
+    ``layers`` holds ``gemm``'s (w, bias, relu, out, start, start_row) per layer;
+    every out but the last is bf16, the next layer's operand."""
     torch = _tm()
+    bf16, f32 = torch.bfloat16, torch.float32
     arr = (_abi.SgDenseLayer * len(layers))()
-    k = x.shape[1]
+    R, k = x.shape
+    ldx, unit = x.stride()
+    if x.dtype is not bf16 or unit != 1:
+        raise ValueError("dense_forward: x must be bf16 with unit column stride")
+    left = len(layers)
     for q, (w, bias, relu, out, start, start_row) in zip(arr, layers):
-        if w.shape[1] != k or out.shape[0] != x.shape[0] or out.shape[1] != w.shape[0]:
+        left -= 1
+        N, K = w.shape
+        (ldw, w_unit), (ldd, unit) = w.stride(), out.stride()
+        half = out.dtype is bf16
+        if K != k or out.shape != (R, N):
             raise ValueError("dense_forward: w (N, K) of the input's K and out (R, N) are needed")
-        q.N, q.K, q.ldw, q.ldd = w.shape[0], k, w.stride(0), out.stride(0)
-        q.d_dtype = _abi.SG_OUT_BF16 if out.dtype == torch.bfloat16 else _abi.SG_OUT_F32
+        if not (w.dtype is bf16 and bias.dtype is f32 and w_unit == 1 and unit == 1 and
+                (half or (left == 0 and out.dtype is f32))):
+            raise ValueError("dense_forward: w and out must be bf16 (the last out may be fp32), bias fp32, "
+                             "w and out with unit column stride")
+        q.N, q.K, q.ldw, q.ldd = N, k, ldw, ldd
+        q.d_dtype = _abi.SG_OUT_BF16 if half else _abi.SG_OUT_F32
         q.relu = 1 if relu else 0
         q.w, q.bias, q.out = w.data_ptr(), bias.data_ptr(), out.data_ptr()
         if start is not None:
+            _start_rows("dense_forward", R, N, start, start_row)
             q.cinit, q.ldc = start.data_ptr(), start.stride(0)
             q.crow = None if start_row is None else start_row.data_ptr()
-        k = q.N
-    _check(lib().sg_dense_forward(x.shape[0], x.data_ptr(), x.stride(0), len(layers), arr, _p(_err(x.device).t),
-                                  _stream(x)), "sg_dense_forward")
+        k = N
+    _check(lib().sg_dense_forward(R, x.data_ptr(), ldx, len(layers), arr, _p(_err(x.device).t), _stream(x)),
+           "sg_dense_forward")
 
 
 def col2im(dcols, shape, kpad, act=None, out=None):
