@@ -84,7 +84,8 @@ int sg_conv_forward(int32_t P, int32_t size, const void* x, int32_t count, const
                     void* stream);
 
 /* A stack of dense layers on x (rows, ldx) bf16, each reading the output of the
- * one before: sg_gemm per layer (sg_gemm_from where cinit is given), in one call. */
+ * one before: sg_gemm per layer (sg_gemm_from where cinit is given), in one call.
+ * Every layer but the last has d_dtype SG_OUT_BF16. */
 typedef struct SgDenseLayer {
     int32_t N, K, ldw, ldd, d_dtype, relu;
     const void* w;

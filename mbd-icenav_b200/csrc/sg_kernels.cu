@@ -1036,6 +1036,8 @@ int sg_conv_forward(int32_t P, int32_t size, const void* x, int32_t count, const
 int sg_dense_forward(int32_t rows, const void* x, int32_t ldx, int32_t count, const SgDenseLayer* layers, int32_t* err,
                      void* stream) {
     if (count < 1 || !layers) return SG_ERR_INVALID;
+    for (int i = 0; i + 1 < count; ++i)  // the next layer's operand
+        if (layers[i].d_dtype != SG_OUT_BF16) return SG_ERR_INVALID;
     for (int i = 0; i < count; ++i) {
         const SgDenseLayer& q = layers[i];
         const int rc = q.cinit ? sg_gemm_from(rows, q.N, q.K, x, ldx, q.w, q.ldw, q.out, q.ldd, q.d_dtype, q.bias, q.relu,

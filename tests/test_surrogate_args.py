@@ -1,5 +1,6 @@
 """The surrogate's batched calls refuse operands of other types, strides and sizes than
 the kernels read, before anything is launched (no GPU: the library is a stand-in)."""
+import ctypes
 from types import SimpleNamespace
 
 import pytest
@@ -94,3 +95,15 @@ def test_weight_grads_refuses(ops, bad):
     with pytest.raises(ValueError):
         ops.grads([tuple(dict(a, **bad).values())])
     assert len(ops.calls) == 1
+
+
+def test_a_middle_layer_of_fp32_is_refused_at_the_c_boundary():
+    """Before the first layer is launched: its pointers are not looked at."""
+    from mbd_icenav_b200 import _abi
+    lib = _abi.load_library()
+    arr = (_abi.SgDenseLayer * 2)()
+    for q in arr:
+        q.N, q.K, q.ldw, q.ldd, q.d_dtype = 64, 64, 64, 64, _abi.SG_OUT_F32
+        q.w = q.out = 16
+    err = ctypes.c_int32()
+    assert lib.sg_dense_forward(128, 16, 64, 2, arr, ctypes.addressof(err), None) == _abi.SG_ERR_INVALID
