@@ -123,8 +123,11 @@ EXPORTS = ("dem_create", "dem_frame_step", "dem_scan_segment", "dem_sync_status"
            "dem_rollout_sweep_features")
 
 def current_stream(device) -> int:
-    """The handle of torch's current stream on ``device`` (a launch argument)."""
+    """The handle of torch's current stream on ``device`` (a launch argument).  A
+    device that is not a GPU is refused: its tensors are not the kernels' to read."""
     import torch
+    if device.type != "cuda":
+        raise ValueError(f"expected a cuda device, but got: {device}")
     i = device.index
     return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if i is None else i)
 
