@@ -234,8 +234,11 @@ int launch_costs(const RcArgs& c, const int32_t* sys_start, const void* eta0, co
             ++g.group_log2;
     const int R = 1 << g.group_log2, threads = R > 1 ? kRcGroupThreads : kRcThreads;
     const size_t smem = sizeof(float) * (words * R + c.H + 1);
+    // The limit belongs to the kernel, not to the call: always the longest horizon's,
+    // so that calls of other threads find room for theirs.
+    constexpr int kMost = (int)sizeof(float) * (rc_stride(kRcMaxHorizon + 1) + kRcMaxHorizon + 1);
     if (smem > 46 * 1024 && cudaFuncSetAttribute(rollout_cost_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 (int)smem) != cudaSuccess)
+                                                 kMost) != cudaSuccess)
         return DEM_ERR_CUDA;
     rollout_cost_kernel<T><<<(c.Q + R - 1) / R, threads, smem, st>>>(g, sys_start, (const T*)eta0, (const T*)eta_hist,
                                                                      (const T*)u, grid, (const T*)masses,
@@ -598,8 +601,10 @@ template <typename T, int G>
 int launch_sweep(const SwArgs& c, const void* eta0, const void* hist, const void* pos, const void* radii,
                  const void* mass, const int32_t* bi, const int32_t* bj, float* out, cudaStream_t st) {
     const size_t smem = SwLayout(G, c.H, c.n).bytes;
+    // the kernel's limit is the largest call's, whatever other threads call
+    const int most = (int)SwLayout(G, kSwMaxHorizon, kSwMaxElements).bytes;
     if (smem > 46 * 1024 && cudaFuncSetAttribute(sweep_kernel<T, G>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 (int)smem) != cudaSuccess)
+                                                 most) != cudaSuccess)
         return DEM_ERR_CUDA;
     sweep_kernel<T, G><<<(c.Q + G - 1) / G, kSwThreads, smem, st>>>(c, (const T*)eta0, (const T*)hist, (const T*)pos,
                                                                     (const T*)radii, (const T*)mass, bi, bj, out);
