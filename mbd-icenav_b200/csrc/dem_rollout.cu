@@ -393,15 +393,21 @@ extern "C" int dem_rollout_ice_terms(int32_t dtype, int32_t n_systems, int32_t h
 // test and the first hit is the lowest bit of the vote.  A CTA takes eight
 // neighbouring candidates, a warp each: their poses are read as rows, and as an
 // element's hits are a byte, a bond is looked up once for all of them.
+// A candidate's sums have one order, whatever the population: those of the elements
+// e, e + 256, ... first, 256 sums, and these in a binary tree, 128 apart first.  A
+// warp that has a candidate alone goes through the eight 32s of elements of each 256
+// one after another, in the order in which the tree joins their sums, and keeps
+// those that wait for their partner in shared memory.
 // (A thread per element, pose after pose, one candidate a CTA: 267 us for 8192
 // candidates of 64 steps through 450 elements and 1500 bonds; the boxes and votes
-// with one candidate a CTA: 84; now 57.)
+// with one candidate a CTA: 85; now 60, 4 of them for the one order of the sums.)
 // ════════════════════════════════════════════════════════════════════════════
 namespace {
 
 constexpr int kSwThreads = 256;
 constexpr int kSwWarps = kSwThreads / 32;
 constexpr int kSwFeatures = DEM_SWEEP_FEATURES;
+constexpr int kSwSums = 5;  // features 1 to 5; the others are counts
 constexpr int kSwMaxElements = DEM_SWEEP_MAX_ELEMENTS;
 constexpr int kSwMaxHorizon = DEM_SWEEP_MAX_HORIZON;
 
@@ -457,31 +463,33 @@ __device__ __forceinline__ SwBox sw_box(const float4* pose, int t0, int t1) {
     return SwBox{o.x, o.y, o.z, o.w, lo_x, hi_x, lo_y, hi_y, turn};
 }
 
-// Shared memory of a CTA with G candidates: poses (x, y, cos, sin), boxes, hits.
+// Shared memory of a CTA with G candidates: poses (x, y, cos, sin), sums (the eight
+// warps' of one candidate, or three that wait in each of eight warps), boxes, hits.
 struct SwLayout {
-    size_t box, hit, bytes;
+    size_t sum, box, hit, bytes;
     __host__ __device__ SwLayout(int G, int H, int n) {
-        box = sizeof(float4) * (size_t)G * (H + 1);
+        sum = sizeof(float4) * (size_t)G * (H + 1);
+        box = sum + sizeof(double) * kSwSums * 32 * (G == 1 ? kSwWarps : 3 * kSwWarps);
         hit = box + (sizeof(SwBox) * (size_t)G * ((H + 32) / 32 + 1) + 15) / 16 * 16;
         bytes = hit + ((size_t)n + 15) / 16 * 16;
     }
 };
 
-// G candidates a CTA, 8 / G warps each.
+// One candidate a CTA, or eight, a warp each.
 template <typename T, int G>
 __global__ void __launch_bounds__(kSwThreads, 4) sweep_kernel(const SwArgs c, const T* __restrict__ eta0,
                                                               const T* __restrict__ hist, const T* __restrict__ pos,
                                                               const T* __restrict__ radii, const T* __restrict__ mass,
                                                               const int* __restrict__ bi, const int* __restrict__ bj,
                                                               float* __restrict__ out) {
-    constexpr int kWarps = kSwWarps / G;
+    static_assert(G == 1 || G == kSwWarps, "a candidate's sums are a CTA's or a warp's");
     extern __shared__ __align__(16) unsigned char sw_smem[];
     const SwLayout at(G, c.H, c.n);
     float4* pose = reinterpret_cast<float4*>(sw_smem);
     SwBox* box = reinterpret_cast<SwBox*>(sw_smem + at.box);
     unsigned char* hit = sw_smem + at.hit;  // a bit per candidate
-    __shared__ double red[kSwWarps][6];
-    __shared__ int bonds[G][2];
+    double* sums = reinterpret_cast<double*>(sw_smem + at.sum);
+    __shared__ int counts[G][3];  // elements hit, bonds with one end hit and with both
     const int H = c.H, W = H + 1, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int q0 = blockIdx.x * G, groups = (H + 32) / 32;
     for (int i = threadIdx.x; i < W * G; i += kSwThreads) {
@@ -492,7 +500,7 @@ __global__ void __launch_bounds__(kSwThreads, 4) sweep_kernel(const SwArgs c, co
         pose[r * W + t] = make_float4((float)p[0], (float)p[1], (float)cs, (float)sn);
     }
     for (int w = threadIdx.x; w < (c.n + 3) / 4; w += kSwThreads) reinterpret_cast<unsigned*>(hit)[w] = 0u;
-    if (threadIdx.x < 2 * G) bonds[threadIdx.x >> 1][threadIdx.x & 1] = 0;
+    if (threadIdx.x < 3 * G) counts[threadIdx.x / 3][threadIdx.x % 3] = 0;
     __syncthreads();
     // boxes of each 32 poses, then of the path
     for (int i = warp; i < G * (groups + 1); i += kSwWarps) {
@@ -501,11 +509,11 @@ __global__ void __launch_bounds__(kSwThreads, 4) sweep_kernel(const SwArgs c, co
         if (lane == 0) box[i] = b;
     }
     __syncthreads();
-    const int r = warp / kWarps;
+    const int r = G == 1 ? 0 : warp;
     const float4* path = pose + r * W;
     const SwBox* boxes = box + r * (groups + 1);
-    double acc[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-    const int first = 32 * (warp % kWarps);
+    // the 32 elements of each 256 that come i-th: the warp's own, or 0, 4, 2, 6, 1, 5, 3, 7
+    auto part = [&](int i) { return 32 * (G == 1 ? warp : (int)(__brev((unsigned)i) >> 29)); };
     auto load = [&](int e, float& x, float& y, float& rad) {
         x = y = rad = 0.0f;
         if (e < c.n) {
@@ -514,57 +522,87 @@ __global__ void __launch_bounds__(kSwThreads, 4) sweep_kernel(const SwArgs c, co
             rad = (float)radii[e];
         }
     };
+    int met = 0;  // elements hit
+    double acc[kSwSums];
+    double* wait = sums + (G == 1 ? 0 : warp * 3 * kSwSums * 32);
     float nx, ny, nr;
-    load(first + lane, nx, ny, nr);
-    for (int e0 = first; e0 < c.n; e0 += 32 * kWarps) {
-        const int e = e0 + lane;
-        const float ex = nx, ey = ny, gl = c.hl + nr, gw = c.hw + nr;
-        load(e + 32 * kWarps, nx, ny, nr);
-        const bool reach = e < c.n && sw_near(boxes[groups], ex, ey, gl, gw);
-        if (!__any_sync(0xffffffffu, reach)) continue;
-        int th = -1;  // the lane's element: the pose that hits it first
-        for (int k = 0; k < groups; ++k) {
-            const bool near = reach && th < 0 && sw_near(boxes[k], ex, ey, gl, gw);
-            unsigned todo = __ballot_sync(0xffffffffu, near);
-            const int t = 32 * k + lane;
-            const float4 p = path[min(t, H)];
-            while (todo) {
-                const int l = __ffs(todo) - 1;
-                todo &= todo - 1;
-                // every lane takes part in the four shuffles
-                const float lx = __shfl_sync(0xffffffffu, ex, l), ly = __shfl_sync(0xffffffffu, ey, l);
-                const float ll = __shfl_sync(0xffffffffu, gl, l), lw = __shfl_sync(0xffffffffu, gw, l);
-                const float dx = lx - p.x, dy = ly - p.y;
-                const float bx = p.z * dx + p.w * dy;
-                const float by = p.z * dy - p.w * dx;
-                const bool in = fabsf(bx) < ll && fabsf(by) < lw && t <= H;
-                const unsigned v = __ballot_sync(0xffffffffu, in);
-                if (v && lane == l) th = 32 * k + __ffs(v) - 1;
+    load(part(0) + lane, nx, ny, nr);
+    for (int i = 0; i < G; ++i) {
+        for (int k = 0; k < kSwSums; ++k) acc[k] = 0.0;
+        for (int e0 = part(i); e0 < c.n; e0 += kSwThreads) {
+            const int e = e0 + lane;
+            const float ex = nx, ey = ny, gl = c.hl + nr, gw = c.hw + nr;
+            int ahead = e0 + kSwThreads;  // the warp's next elements
+            for (int j = i + 1; j < G && ahead >= c.n; ++j) ahead = part(j);
+            load(ahead + lane, nx, ny, nr);
+            const bool reach = e < c.n && sw_near(boxes[groups], ex, ey, gl, gw);
+            if (!__any_sync(0xffffffffu, reach)) continue;
+            int th = -1;  // the lane's element: the pose that hits it first
+            for (int k = 0; k < groups; ++k) {
+                const bool near = reach && th < 0 && sw_near(boxes[k], ex, ey, gl, gw);
+                unsigned todo = __ballot_sync(0xffffffffu, near);
+                const int t = 32 * k + lane;
+                const float4 p = path[min(t, H)];
+                while (todo) {
+                    const int l = __ffs(todo) - 1;
+                    todo &= todo - 1;
+                    // every lane takes part in the four shuffles
+                    const float lx = __shfl_sync(0xffffffffu, ex, l), ly = __shfl_sync(0xffffffffu, ey, l);
+                    const float ll = __shfl_sync(0xffffffffu, gl, l), lw = __shfl_sync(0xffffffffu, gw, l);
+                    const float dx = lx - p.x, dy = ly - p.y;
+                    const float bx = p.z * dx + p.w * dy;
+                    const float by = p.z * dy - p.w * dx;
+                    const bool in = fabsf(bx) < ll && fabsf(by) < lw && t <= H;
+                    const unsigned v = __ballot_sync(0xffffffffu, in);
+                    if (v && lane == l) th = 32 * k + __ffs(v) - 1;
+                }
+            }
+            met += __popc(__ballot_sync(0xffffffffu, th >= 0));
+            if (th >= 0) {
+                const float4 p = path[th];
+                // the first step's velocity at the start pose
+                const float4 pa = path[max(th, 1)], pb = path[max(th, 1) - 1];
+                const float dx = ex - p.x, dy = ey - p.y;
+                const double m = (double)mass[e];
+                const double vx = (double)((pa.x - pb.x) * c.inv_dt), vy = (double)((pa.y - pb.y) * c.inv_dt);
+                const double dd = sqrt((double)dx * (double)dx + (double)dy * (double)dy);
+                const double vn = fmax(0.0, (vx * (double)dx + vy * (double)dy) / fmax(dd, 1e-6));
+                acc[0] += m;
+                acc[1] += 0.5 * m * (vx * vx + vy * vy);
+                acc[2] += m * vn;
+                acc[3] += m * (double)(H + 1 - th) / (double)(H + 1);
+                acc[4] += 0.5 * m * vn * vn;
+                atomicOr(reinterpret_cast<unsigned*>(hit) + (e >> 2), (1u << r) << (8 * (e & 3)));
             }
         }
-        if (th >= 0) {
-            const float4 p = path[th];
-            // the first step's velocity at the start pose
-            const float4 pa = path[max(th, 1)], pb = path[max(th, 1) - 1];
-            const float dx = ex - p.x, dy = ey - p.y;
-            const double m = (double)mass[e];
-            const double vx = (double)((pa.x - pb.x) * c.inv_dt), vy = (double)((pa.y - pb.y) * c.inv_dt);
-            const double dd = sqrt((double)dx * (double)dx + (double)dy * (double)dy);
-            const double vn = fmax(0.0, (vx * (double)dx + vy * (double)dy) / fmax(dd, 1e-6));
-            acc[0] += 1.0;
-            acc[1] += m;
-            acc[2] += 0.5 * m * (vx * vx + vy * vy);
-            acc[3] += m * vn;
-            acc[4] += m * (double)(H + 1 - th) / (double)(H + 1);
-            acc[5] += 0.5 * m * vn * vn;
-            atomicOr(reinterpret_cast<unsigned*>(hit) + (e >> 2), (1u << r) << (8 * (e & 3)));
+        if (G > 1) {
+            // join the sums that wait for this one, as a binary counter carries
+            int b = 0;
+            for (; (i >> b) & 1; ++b)
+                for (int k = 0; k < kSwSums; ++k) acc[k] = wait[(b * kSwSums + k) * 32 + lane] + acc[k];
+            if (b < 3)
+                for (int k = 0; k < kSwSums; ++k) wait[(b * kSwSums + k) * 32 + lane] = acc[k];
         }
     }
-    for (int k = 0; k < 6; ++k) {
-        for (int d = 16; d > 0; d >>= 1) acc[k] += __shfl_down_sync(0xffffffffu, acc[k], d);
-        if (lane == 0) red[warp][k] = acc[k];
+    auto lanes = [&](double v) {
+        for (int d = 16; d > 0; d >>= 1) v += __shfl_down_sync(0xffffffffu, v, d);
+        return v;
+    };
+    if (lane == 0) atomicAdd(&counts[r][0], met);
+    if (G > 1) {
+        for (int k = 0; k < kSwSums; ++k) {
+            const double v = lanes(acc[k]);
+            if (lane == 0 && q0 + r < c.Q) out[(size_t)(q0 + r) * kSwFeatures + 1 + k] = (float)v;
+        }
+    } else {
+        for (int k = 0; k < kSwSums; ++k) sums[(warp * kSwSums + k) * 32 + lane] = acc[k];
     }
     __syncthreads();
+    if (G == 1 && warp < kSwSums) {
+        auto of = [&](int w) { return sums[(w * kSwSums + warp) * 32 + lane]; };
+        const double v = lanes(((of(0) + of(4)) + (of(2) + of(6))) + ((of(1) + of(5)) + (of(3) + of(7))));
+        if (lane == 0) out[(size_t)q0 * kSwFeatures + 1 + warp] = (float)v;
+    }
     constexpr int kAhead = 4;  // bonds whose ends are read before the first is looked up
     for (int b0 = threadIdx.x; b0 < c.nb; b0 += kAhead * kSwThreads) {
         int i[kAhead], j[kAhead];
@@ -580,22 +618,17 @@ __global__ void __launch_bounds__(kSwThreads, 4) sweep_kernel(const SwArgs c, co
             const unsigned hi = hit[i[k]], hj = hit[j[k]];
             for (unsigned x = hi | hj; x; x &= x - 1) {  // few: the candidates that hit an end
                 const int l = __ffs(x) - 1;
-                atomicAdd(&bonds[l][((hi & hj) >> l) & 1u], 1);
+                atomicAdd(&counts[l][1 + (((hi & hj) >> l) & 1u)], 1);
             }
         }
     }
     __syncthreads();
-    if (threadIdx.x < G * kSwFeatures) {
-        const int l = threadIdx.x / kSwFeatures, k = threadIdx.x % kSwFeatures;
-        double v = 0.0;
-        if (k < 6)
-            for (int w = 0; w < kWarps; ++w) v += red[l * kWarps + w][k];
-        else
-            v = (double)bonds[l][k - 6];
-        if (q0 + l < c.Q) out[(size_t)(q0 + l) * kSwFeatures + k] = (float)v;
+    if (threadIdx.x < 3 * G) {
+        const int l = threadIdx.x / 3, k = threadIdx.x % 3;
+        if (q0 + l < c.Q) out[(size_t)(q0 + l) * kSwFeatures + (k == 0 ? 0 : 5 + k)] = (float)counts[l][k];
     }
 }
-static_assert(kSwFeatures == 8 && kSwWarps * kSwFeatures <= kSwThreads, "a thread per feature of a candidate");
+static_assert(kSwFeatures == 8 && kSwThreads == 256, "the order of a candidate's sums");
 
 template <typename T, int G>
 int launch_sweep(const SwArgs& c, const void* eta0, const void* hist, const void* pos, const void* radii,
@@ -612,8 +645,9 @@ int launch_sweep(const SwArgs& c, const void* eta0, const void* hist, const void
 }
 
 // Eight candidates a CTA from the population on whose CTAs fill the SMs: 2368
-// candidates in 27 us against 29 with one a CTA, 8192 in 57 against 80; below, 1184
-// in 29 against 19 and 64 in 23 against 9.
+// candidates in 29 us either way, 4736 in 37 against 52 with one a CTA, 8192 in 60
+// against 85; below, 1776 in 27 against 24.5, 1184 in 27 against 18 and 64 in 22
+// against 11.
 constexpr int kSwGroupFrom = 148 * 16;
 
 }  // namespace
