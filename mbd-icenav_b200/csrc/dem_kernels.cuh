@@ -2075,9 +2075,10 @@ __device__ __forceinline__ bool contact_term(const ForceConst<T>& fc, bool h15, 
 }
 
 // The same two terms without branches, for code that computes them for every
-// lane and selects afterwards.  Each returns the same bits as the form above
-// when it leaves `ok` set; with `ok` cleared (an operand outside the fast range,
-// or an undecided rounding) the caller takes the form above.
+// lane and selects afterwards.  Each returns the same bits as the form above (but
+// for the sign of a zero, which the sums take no notice of) when it leaves `ok`
+// set; with `ok` cleared (an operand outside the fast range, or an undecided
+// rounding) the caller takes the form above.
 template <typename T>
 __device__ __forceinline__ void bond_term_nr(const SlotRec<T>& r, typename vec2_of<T>::type kb, T ex, T ey, T& fx,
                                              T& fy, T& cr, bool& ok) {

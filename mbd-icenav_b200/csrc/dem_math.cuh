@@ -80,16 +80,19 @@ __device__ __forceinline__ double jsin(double a) { return sin(a); }
 
 // ─── correctly rounded division and square root without branches ────────────
 // Newton iterations from the hardware's seed and Markstein's final steps
-// (P. Markstein, IBM J. Res. Dev. 34, 1990): with y close to 1/d and q within an
-// ulp of x/d, the exact remainder e = x - q d gives x/d rounded to nearest as
-// q + e y; with g within an ulp of sqrt(x) and h close to 1/(2 sqrt(x)), the
-// exact x - g^2 gives the root rounded to nearest as g + (x - g^2) h.  Equal to
-// the operators' results bit for bit (checked for every float significand of the
-// root, and on 7e9 random and edge significands of each division) while operands stay
-// within kFastLo..kFastHi, where no remainder underflows; callers test that and
-// leave the rest to the operators.  One after another, the operators' range
-// checks and branches are what a substep of a single warp waits for: a block
-// of these interleaves instead, and a reciprocal serves several quotients.
+// (P. Markstein, IBM J. Res. Dev. 34, 1990): with y = 1/d rounded to nearest and q
+// within an ulp of x/d, the exact remainder e = x - q d gives x/d rounded to nearest
+// as q + e y; an iteration from a y within an ulp of 1/d rounds it to nearest unless
+// d's significand is all ones.  With g within an ulp of sqrt(x) and h close to
+// 1/(2 sqrt(x)), the exact x - g^2 gives the root rounded to nearest as g + (x - g^2) h.
+// The operators' values while operands stay within kFastLo..kFastHi, where no
+// remainder underflows, or the numerator is zero (the quotient's sign is then not the
+// operator's: callers add it to sums, which it does not change); callers test that
+// and leave the rest to the operators.  tests/test_gpu_fast_math.py compares them:
+// every float significand of the root, the roots and quotients closest to half way
+// between two results, 2^30 random and edge operands of each.  One after another, the
+// operators' range checks and branches are what a substep of a single warp waits
+// for: a block of these interleaves instead, and a reciprocal serves several quotients.
 template <typename T> struct FastRange;
 template <> struct FastRange<float> {
     static __device__ __forceinline__ float lo() { return 8.6736174e-19f; }  // 2^-60
@@ -99,7 +102,7 @@ template <> struct FastRange<double> {
     static __device__ __forceinline__ double lo() { return 3.8725919148493183e-121; }  // 2^-400
     static __device__ __forceinline__ double hi() { return 2.5822498780869086e120; }   // 2^400
 };
-// a numerator or divisor that the fast forms may take (a zero numerator is exact)
+// a numerator or divisor that the fast forms may take
 template <typename T> __device__ __forceinline__ bool fast_ok(T x) {
     const T ax = fabs(x);
     return ax >= FastRange<T>::lo() && ax <= FastRange<T>::hi();
@@ -114,8 +117,13 @@ __device__ __forceinline__ float rcp_nr(float d) {
 __device__ __forceinline__ double rcp_nr(double d) {
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+    const double e = fma(-d, y, 1.0);  // 2^-19 at most: e + e^2 leaves 2^-57
+    y = fma(fma(e, e, e), y, y);
     y = fma(fma(-d, y, 1.0), y, y);
-    return fma(fma(-d, y, 1.0), y, y);
+    // 2^k (1 - 2^-53): 1/d is half way and a little more above 2^-k, where y has stayed
+    constexpr long long kOnes = 0xfffffffffffffll;
+    const bool ones = (__double_as_longlong(d) & kOnes) == kOnes;
+    return __longlong_as_double(__double_as_longlong(y) + (ones ? 1 : 0));
 }
 // x / d with y = rcp_nr(d)
 __device__ __forceinline__ float div_nr(float x, float d, float y) {
