@@ -567,6 +567,8 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_kernel(const __grid_const
 }
 
 // ─── glue kernels ───────────────────────────────────────────────────────────
+// The rows of the kernels below are counted in unsigned: up to 2^31 of them and a
+// step of the grid beyond stay in range.
 // im2col for channel counts that are multiples of 8: a thread per 16-byte chunk of
 // a patch row, which lies within one tap.  blockDim.x is the chunks of a row, so
 // that a thread's tap and channel stay the same and its rows advance.  The
@@ -577,8 +579,8 @@ __global__ void im2col8_kernel(int rows, int H, int W, int C, const __nv_bfloat1
     const unsigned Ho = H / 2, Wo = W / 2;
     const int k = threadIdx.x * 8, t = k / C, c = k % C, ky = t / 3, kx = t % 3;
     const bool live = k < 9 * C;
-    for (int r = blockIdx.x * blockDim.y + threadIdx.y; r < rows; r += gridDim.x * blockDim.y) {
-        const unsigned ox = (unsigned)r % Wo, q = (unsigned)r / Wo, oy = q % Ho, b = q / Ho;
+    for (unsigned r = blockIdx.x * blockDim.y + threadIdx.y; r < (unsigned)rows; r += gridDim.x * blockDim.y) {
+        const unsigned ox = r % Wo, q = r / Wo, oy = q % Ho, b = q / Ho;
         const int iy = 2 * (int)oy - 1 + ky, ix = 2 * (int)ox - 1 + kx;
         uint4 v = make_uint4(0u, 0u, 0u, 0u);
         if (live && iy >= 0 && iy < H && ix >= 0 && ix < W)
@@ -592,12 +594,12 @@ __global__ void im2col1_kernel(int rows, int H, int W, const __nv_bfloat16* __re
                                __nv_bfloat16* __restrict__ cols) {
     const unsigned Ho = H / 2, Wo = W / 2;
     const int k = threadIdx.x * 8;
-    for (int r = blockIdx.x * blockDim.y + threadIdx.y; r < rows; r += gridDim.x * blockDim.y) {
+    for (unsigned r = blockIdx.x * blockDim.y + threadIdx.y; r < (unsigned)rows; r += gridDim.x * blockDim.y) {
         __align__(16) __nv_bfloat16 v[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j) v[j] = __float2bfloat16_rn(0.0f);
         if (k < 9) {
-            const unsigned ox = (unsigned)r % Wo, q = (unsigned)r / Wo, oy = q % Ho, b = q / Ho;
+            const unsigned ox = r % Wo, q = r / Wo, oy = q % Ho, b = q / Ho;
             const __nv_bfloat16* img = X + (size_t)b * H * W;
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
@@ -616,8 +618,8 @@ __global__ void col2im8_kernel(int pixels, int H, int W, int C, const float* __r
                                const __nv_bfloat16* __restrict__ act, __nv_bfloat16* __restrict__ dX) {
     const unsigned Ho = H / 2, Wo = W / 2;
     const int c = threadIdx.x * 8;
-    for (int p = blockIdx.x * blockDim.y + threadIdx.y; p < pixels; p += gridDim.x * blockDim.y) {
-        const unsigned ix = (unsigned)p % W, q = (unsigned)p / W, iy = q % H, b = q / H;
+    for (unsigned p = blockIdx.x * blockDim.y + threadIdx.y; p < (unsigned)pixels; p += gridDim.x * blockDim.y) {
+        const unsigned ix = p % W, q = p / W, iy = q % H, b = q / H;
         float s[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
         for (int ky = 0; ky < 3; ++ky) {
             const int ty = (int)iy + 1 - ky;
@@ -848,7 +850,7 @@ __global__ void mse_kernel(int rows, int n_out, const float* __restrict__ pred, 
     if (blockDim.x % ldg == 0) {
         // whole rows a step: the same entries for every thread without a division each
         const int c = threadIdx.x % ldg, step = blockDim.x / ldg;
-        for (int r = threadIdx.x / ldg; r < rows; r += step) entry(r, c);
+        for (unsigned r = threadIdx.x / ldg; r < (unsigned)rows; r += step) entry((int)r, c);
     } else {
         const long long total = (long long)rows * ldg;
         for (long long i = threadIdx.x; i < total; i += blockDim.x) entry((int)(i / ldg), (int)(i % ldg));
@@ -887,8 +889,8 @@ __global__ void pack_rows_kernel(int rows, int enc_dim, const __nv_bfloat16* __r
 __global__ void pack_rows8_kernel(int rows, int enc_dim, const __nv_bfloat16* __restrict__ enc, int ld_enc,
                                   const int* __restrict__ enc_row, int n_extra, const float* __restrict__ extra,
                                   int ld_extra, __nv_bfloat16* __restrict__ x, int ldx) {
-    for (int r = blockIdx.x * blockDim.y + threadIdx.y; r < rows; r += gridDim.x * blockDim.y) {
-        const __nv_bfloat16* er = enc ? enc + (size_t)(enc_row ? enc_row[r] : r) * ld_enc : nullptr;
+    for (unsigned r = blockIdx.x * blockDim.y + threadIdx.y; r < (unsigned)rows; r += gridDim.x * blockDim.y) {
+        const __nv_bfloat16* er = enc ? enc + (size_t)(enc_row ? enc_row[r] : (int)r) * ld_enc : nullptr;
         for (int c = threadIdx.x * 8; c < ldx; c += blockDim.x * 8) {
             uint4 v = make_uint4(0u, 0u, 0u, 0u);
             if (c < enc_dim) {
