@@ -1,8 +1,9 @@
 """Autotuner of the batched rollouts' work split.
 
 How a substep's work is split over the persistent grid is a runtime choice of
-the handle (``dem_set_work_split``): a thread or a warp per active element,
-and a CTA or a warp per list rebuild / escaped element.  Every choice gives
+the handle (``dem_set_work_split``): a thread per active element or lanes that
+share one (from shared memory while it holds the active elements), and a CTA or
+a warp per list rebuild / escaped element.  Every choice gives
 bit-identical results (the GPU tests check each one against the others), so
 the fastest can be picked by measurement alone.  ``tune`` times each choice on
 the caller's own batch with CUDA events (median of a few runs) and sets the

@@ -7,22 +7,28 @@
 // execute the same device functions, so they give identical results.
 //
 // Phases of a frame (reference: medea_ice_ship/jax_simulation.py:397-699)
-//   P_CONTACT  ship contact (jax_geometry.py:515-594), contact force, side push,
-//              submergence + buoyancy (jax_simulation.py:431-496), floe
-//              collision flags, crack-front flags, grid insert for the
-//              neighbour list, per-chunk partial sums for the thrust cap
+//   P_CULL     elements near the hull, escapes from the neighbour lists' margins,
+//              compaction of the grid's buckets
+//   P_NEAR     ship contact of the near elements (jax_geometry.py:515-594); beside
+//              it the escaped elements' new references
+//   P_CFORCE   contact force, side push, submergence + buoyancy
+//              (jax_simulation.py:431-496), floe collision flags, per-chunk partial
+//              sums for the thrust cap; beside it the rebuild of marked lists
 //   P_REDUCE   fixed-order reduction of the partials -> thrust scale, reaction
 //              on the ship, vessel step (jax_vessel_dynamics.py:246-348),
-//              floe activation and DPDEM eligibility (jax_simulation.py:498-524),
-//              neighbour-list build
+//              floe activation (jax_simulation.py:498-524), crack-front flags and
+//              bond slot records of the active elements
 //   per substep s (jax_simulation.py:363-395, 527-532):
-//     P_INSERT / P_NBR   neighbour-list rebuild (skipped while the Verlet skin holds)
+//     escape, build_all   neighbour lists of elements that left their margin within
+//               the frame, or of all (skipped otherwise)
 //     P_FORCE   fused bond forces + ice-ice contact + drag + rotational drag +
-//               semi-implicit integration, one thread per element, gather form
+//               semi-implicit integration of the active elements, in gather form
 //               (no atomics: each element sums its own bond and contact terms in
-//               the reference's scatter order)
-//   P_FRACTURE crack front, DPDEM damage, collision breaks (jax_simulation.py:534-653)
-//              and history rows
+//               the reference's scatter order); all substeps in one go with the
+//               elements in shared memory while it holds them, else by groups of
+//               lanes or a thread per element
+//   P_FRACTURE crack front, DPDEM damage, collision breaks (jax_simulation.py:534-653),
+//              DPDEM eligibility and history rows
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -461,9 +467,11 @@ __device__ __forceinline__ int sys_id(const KArgs<T>& a, int e) {
 // What this is for: with the lists kept up inside the substeps (re-referencing
 // at the even ones, rebuilding at the odd ones) a force phase was as long as a
 // rebuild and the element's force after it, 10 us, and with one margin for all
-// a frame of the 12k-element field had 1.7 escape phases.  Now a force phase
-// there takes 7.8 us and one frame in five has an escape phase: 149 -> 122 us
-// a frame; the 237k-element pack 205 -> 150 us, all of it active 842 -> 750 us.
+// a frame of the 12k-element field had 1.7 escape phases.  With the upkeep beside
+// the ship contact, and the elements' loads as they were, a force phase there took
+// 7.8 us and one frame in five had an escape phase: 149 -> 122 us a frame; the
+// 237k-element pack 205 -> 150 us, all of it active 842 -> 750 us.  (With the
+// elements in shared memory a substep is 3.5 to 4.4 us and such a frame 81.)
 
 template <typename T>
 __device__ __forceinline__ bool escaped_from(T px, T py, T rx, T ry, T h) {
@@ -1005,7 +1013,6 @@ __device__ void upkeep_build(const KArgs<T>& a, int nd) {
     if (a.mark_split == DEM_SPLIT_CTA || (a.mark_split == DEM_SPLIT_AUTO && nd <= 2 * (int)gridDim.x)) {
         for (int q = gridDim.x - 1 - blockIdx.x; q < nd; q += gridDim.x) block_build(a, a.dirty_list[q]);
     } else {
-        const int wl = threadIdx.x >> 5;
         const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
         const int nwarps = (gridDim.x * blockDim.x) >> 5;
         for (int q = warp; q < nd; q += nwarps) warp_build(a, a.dirty_list[q]);
@@ -1016,7 +1023,6 @@ __device__ void upkeep_build(const KArgs<T>& a, int nd) {
 // Rebuild every list (when most elements escaped at once).
 template <typename T>
 __device__ void phase_build_all(const KArgs<T>& a, int nblk) {
-    const int wl = threadIdx.x >> 5;
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nwarps = (nblk * blockDim.x) >> 5;
     for (int e = warp; e < a.n; e += nwarps) warp_build(a, e);
@@ -1932,11 +1938,11 @@ __device__ void phase_reduce(const KArgs<T>& a, const Frame<T>& F, bool upkept) 
 }
 
 // ─── P_FORCE: one substep (jax_simulation.py:63-268, 363-395) ───────────────
-// One thread per element, gather form: each element sums its own bond and
-// contact terms in the reference's scatter order, so no atomics are needed.
-// Positions are packed with radii as {x, y, r} (one 16-byte load per neighbour,
-// velocities only for overlapping pairs) and bond slots are 16-byte records;
-// the loads of a batch are issued before any of them is used.
+// Gather form: each element, a thread's or a group of lanes', sums its own bond
+// and contact terms in the reference's scatter order, so no atomics are needed.
+// Positions are packed with radii as {x, y, r, r^3} (one 16-byte load per
+// neighbour) and bond slots are 16-byte records; the loads of a batch are issued
+// before any of them is used.
 // Every operation is unfused (-fmad=false) and in the reference's order, with
 // divisions where it divides, so that fp32 forces round as NumPy's fp32
 // evaluation of the same expressions does.
@@ -2500,7 +2506,6 @@ __device__ void phase_force(const KArgs<T>& a, const Frame<T>& F, int s, unsigne
         }
     } else if (has_dirty) {
         // one warp rebuilds the list, then computes the element
-        const int wl = threadIdx.x >> 5;
         for (int q = warp; q < nd; q += nwarps) {
             const int e = a.dirty_list[q];
             warp_build(a, e);
