@@ -108,28 +108,22 @@ def gemm(A, B, out=None, bias=None, relu=False, mask=None, out_dtype=None, start
     return out
 
 
-def _operands(name, *ts):
-    """What every tensor-core operand has to be."""
-    bf16 = _tm().bfloat16
-    for t in ts:
-        if t.dtype != bf16 or t.stride(-1) != 1:
-            raise ValueError(f"{name}: operands must be bf16 with unit column stride")
-
-
 def weight_grads(layers):
     """For every (dy, x, g, gb) of ``layers``, in one launch: g (N, K) fp32 = dy.T @ x
     and gb (N,) fp32 = column sums of dy, for dy (R, N) and x (R, K) bf16."""
     torch = _tm()
+    bf16, f32 = torch.bfloat16, torch.float32
     arr = (_abi.SgWeightGrad * len(layers))()
     for q, (dy, x, g, gb) in zip(arr, layers):
-        _operands("weight_grads", dy, x)
-        if g.dtype != torch.float32 or gb.dtype != torch.float32 or not gb.is_contiguous():
-            raise ValueError("weight_grads: g and gb must be fp32, gb contiguous")
-        q.R, q.N = dy.shape
-        q.K = x.shape[1]
-        if x.shape[0] != q.R or tuple(g.shape) != (q.N, q.K) or not g.is_contiguous() or gb.numel() != q.N:
-            raise ValueError("weight_grads: dy (R, N), x (R, K), g (N, K) contiguous and gb (N,) are needed")
-        q.ldy, q.ldx = dy.stride(0), x.stride(0)
+        R, N = dy.shape
+        rows, K = x.shape
+        (ldy, y_unit), (ldx, x_unit) = dy.stride(), x.stride()
+        if rows != R or g.shape != (N, K) or not g.is_contiguous() or gb.numel() != N or not gb.is_contiguous():
+            raise ValueError("weight_grads: dy (R, N), x (R, K), g (N, K) and gb of N, both contiguous, are needed")
+        if not (dy.dtype is bf16 and x.dtype is bf16 and y_unit == 1 and x_unit == 1 and g.dtype is f32 and
+                gb.dtype is f32):
+            raise ValueError("weight_grads: dy and x must be bf16 with unit column stride, g and gb fp32")
+        q.R, q.N, q.K, q.ldy, q.ldx = R, N, K, ldy, ldx
         q.dY, q.X, q.G, q.gb = dy.data_ptr(), x.data_ptr(), g.data_ptr(), gb.data_ptr()
     dy = layers[0][0]
     _check(lib().sg_weight_grads(len(layers), arr, _p(_err(dy.device).t), _stream(dy)), "sg_weight_grads")
