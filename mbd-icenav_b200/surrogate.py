@@ -190,14 +190,18 @@ class SurrogateNet:
         """MLP on rows [enc[enc_row[r]] | extra[r]] -> (R, OUT_ROWS) fp32 (first N_OUT columns live)."""
         torch = _tm()
         R = int(extra.shape[0])
+        if enc_row is not None and (enc_row.dtype is not torch.int32 or not enc_row.is_contiguous()):
+            enc_row = enc_row.to(torch.int32).contiguous()
         # Rows that share encoder rows (a plan's population shares one patch) share
         # the encoder's part of the first layer: it is summed once per encoder row
         # and each head row goes on from there, the same sums in the same order.
         # For 8192 rows on one patch that leaves 256 of the layer's 2304 input
         # columns per row; with more than a quarter as many encoder rows as head
-        # rows the separate product no longer pays.
+        # rows the separate product no longer pays.  (The product reads the encoder
+        # rows by TMA, which wants them on 16-byte boundaries.)
         E = enc_dim()
-        shared = not keep and enc_row is not None and 4 * int(enc.shape[0]) <= R
+        shared = (not keep and enc_row is not None and 4 * int(enc.shape[0]) <= R and enc.stride(0) % 8 == 0
+                  and enc.data_ptr() % 16 == 0)
         if shared:
             first = self._buf(f"{tag}_e", (int(enc.shape[0]), HIDDEN), torch.float32)
             ops.gemm(enc, self.fc[0].w[:, :E], out=first)
